@@ -1125,7 +1125,7 @@ __global__ void __launch_bounds__(CF_THREADS, sizeof(T) == 4 && NZM <= 20 ? 4 : 
         add_totals(s_t, acc, slot_e, slot_e2);
     }
     extern __shared__ float4 s_dyn4[];
-    T4 *s_co = (T4 *)s_dyn4;   // [CF_COLS][zn], and NZM entries that a short last row may run into
+    T4 *s_co = (T4 *)s_dyn4;   // [CF_COLS][zn], and NZM entries that the last row's loads may run into
     __shared__ int4 s_col[CF_COLS];
     const int i = blockIdx.x * CF_THREADS + threadIdx.x;
     const bool own = i < n;
@@ -1141,10 +1141,13 @@ __global__ void __launch_bounds__(CF_THREADS, sizeof(T) == 4 && NZM <= 20 ? 4 : 
     const double2 y1 = col_phase(pf, 0, 1);
     double2 xy = make_double2(0, 0);
     int pnx = -1, pny = 0;
-    for (int e = threadIdx.x; e < NZM; e += CF_THREADS) {
+    // zero all over: where a range's first group holds fewer than CF_COLS
+    // columns, the loads past its last row meet rows that no group has filled,
+    // and a zero of Z times what shared memory held before may be NaN
+    for (int e = threadIdx.x; e < CF_COLS * zn + NZM; e += CF_THREADS) {
         T4 o;
         o.x = o.y = o.z = o.w = 0;
-        s_co[CF_COLS * zn + e] = o;
+        s_co[e] = o;
     }
     const T kz1 = (T)vz, kz2 = (T)(vz * vz), kz3 = (T)(vz * vz * vz);
     double D1[3] = {0, 0, 0}, D2[6] = {0, 0, 0, 0, 0, 0}, D3[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};

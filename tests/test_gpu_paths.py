@@ -142,3 +142,28 @@ def test_ewald_pair_range(alpha):
     rms = lambda x: np.sqrt((x ** 2).mean())   # noqa: E731
     assert rms(f[1] - f[0]) < 2e-6 * rms(f[0]) + 1e-8   # forces are held in 2^-32
     ens.close()
+
+
+# k sets of a few columns, whose rows are shorter than one batch of the force
+# pass's loads, after a kernel that leaves NaN in the multiprocessors' shared
+# memory (a product of NaN matrices): what a load finds past the last column's
+# row must not enter.  Bounds as in test_multipole_columns
+@pytest.mark.parametrize("kmax", [2, 3])
+def test_multipole_columns_few(kmax):
+    import torch
+    s = systems.polarizable_water(nmol=1331, cutoff=0.9, switch=0.8, kmax=kmax, seed=7)
+    nan = torch.full((4096, 4096), float("nan"), dtype=torch.float64, device="cuda")
+    ens = engine.GpuEnsemble(s)
+    ens.set_reference_forms(True)
+    fr, er, wr = ens.compute_forces(L.TERM_MP_LONG)
+    for precision, tol in (("fp64", 1e-10), ("mixed", 1e-6)):
+        ens.set_precision(precision)
+        ens.set_reference_forms(False)
+        nan @ nan
+        torch.cuda.synchronize()
+        f, e, w = ens.compute_forces(L.TERM_MP_LONG)
+        assert np.isfinite(f).all()
+        assert rms_rel(f, fr) < tol
+        assert abs(e[L.E_LONG] - er[L.E_LONG]) <= tol * abs(er[L.E_LONG])
+        assert np.abs(w - wr).max() < tol * np.abs(wr).max()
+    ens.close()
