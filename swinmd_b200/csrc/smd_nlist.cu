@@ -208,7 +208,9 @@ __device__ __forceinline__ double ref_r2(const double4 &a, const double4 &b, con
 // reference's.  When some site is farther than 0.75 L from the origin
 // (uploaded unwrapped), every candidate takes the FP64 test: the reference's
 // minimum image takes a bounded number of steps and none inside a cell,
-// which matches the integer one only for sites in or near the box.
+// which matches the integer one only for sites in or near the box.  That is
+// settled before the first test, by k_cells or (without cells) by every block
+// for itself, so that both rows of a pair follow the same rule.
 // Instruction issue bounds the pass, and most candidates are beyond the
 // radius (92 % for water in 3 x 3 x 3 cells), hence the skips.  Against one
 // FP64 test per candidate: 6480 sites of water 212 -> 98 us, 12288 sites 340 ->
@@ -222,7 +224,6 @@ __global__ void __launch_bounds__(NB_SITES * 32, 5) k_build(BuildArgs a) {
     __shared__ float s_lo[3][NB_STAGE / 32], s_hi[3][NB_STAGE / 32];   // chunk boxes about the group's first site
     __shared__ int s_off[NB_CELLS + 1], s_cs[NB_CELLS], s_nc[NB_CELLS];
     __shared__ int4 s_c;                 // the group's first site
-    __shared__ int s_far;
     const Box box = a.dbox ? *a.dbox : a.box;
     const double delta = LE ? *a.le : 0.0;
     const unsigned dfrac = LE ? le_frac(delta, box.inv[0]) : 0u;
@@ -230,7 +231,13 @@ __global__ void __launch_bounds__(NB_SITES * 32, 5) k_build(BuildArgs a) {
     const float sx = (float)(box.L[0] / 4294967296.0), sy = (float)(box.L[1] / 4294967296.0),
                 sz = (float)(box.L[2] / 4294967296.0);
     const int ngroup = a.group ? *a.ngroup : (a.n + NB_SITES - 1) / NB_SITES;
-    const bool far_grid = a.group && a.flags[5];
+    bool far = false;
+    if (a.group) {
+        far = a.flags[5];
+    } else {
+        for (int j = threadIdx.x; j < a.n; j += NB_SITES * 32) far = far || far_out(a.pos4[j], box);
+        far = __syncthreads_or(far);
+    }
     for (int gi = blockIdx.x; gi < ngroup; gi += gridDim.x) {
         const int2 grp = a.group ? a.group[gi] : make_int2(-1, gi * NB_SITES);
         const int c = grp.x;
@@ -275,10 +282,7 @@ __global__ void __launch_bounds__(NB_SITES * 32, 5) k_build(BuildArgs a) {
             e1 = a.excl_off[i + 1];
             if (lane == 0) a.disp4[i] = make_double4(0, 0, 0, 0);
         }
-        if (threadIdx.x == 0) {
-            s_c = fi;
-            s_far = far_grid;   // without cells the stages raise it
-        }
+        if (threadIdx.x == 0) s_c = fi;
         __syncthreads();
         if (a.group && threadIdx.x == 0) {
             s_off[0] = 0;
@@ -307,10 +311,8 @@ __global__ void __launch_bounds__(NB_SITES * 32, 5) k_build(BuildArgs a) {
                     // reference does (CellManager.cpp:246-262)
                     same = s_nc[t] == c ? (int)0x80000000 : 0;
                 } else {
-                    const double4 p = a.pos4[j];
-                    q = site_frac(p, box, LE, delta);
+                    q = site_frac(a.pos4[j], box, LE, delta);
                     q.w = j;
-                    if (far_out(p, box)) s_far = 1;
                 }
                 s_m[f] = a.mol[q.w] | same;
                 const int x0 = __shfl_sync(0xffffffffu, q.x, 0), y0 = __shfl_sync(0xffffffffu, q.y, 0),
@@ -330,7 +332,6 @@ __global__ void __launch_bounds__(NB_SITES * 32, 5) k_build(BuildArgs a) {
             }
             __syncthreads();
             if (i < 0) continue;
-            const bool far = s_far;
             const float hi = far ? 3.4e38f : (float)(a.rl2 * (1.0 + 1e-5)), lo = far ? -1.f : (float)(a.rl2 * (1.0 - 1e-5));
             // lane ch: how far chunk ch's box stays from the site (periodic;
             // under shear x is left out, its images slide)

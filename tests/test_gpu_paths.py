@@ -167,3 +167,23 @@ def test_multipole_columns_few(kmax):
         assert abs(e[L.E_LONG] - er[L.E_LONG]) <= tol * abs(er[L.E_LONG])
         assert np.abs(w - wr).max() < tol * np.abs(wr).max()
     ens.close()
+
+
+# a box without cells and more sites than one stage of the build, one of the
+# late ones uploaded 10 boxes away: the minimum image takes 8 steps at most
+# (which leaves it 2 boxes from everything), in both rows of every pair
+@pytest.mark.parametrize("site", [3, 1300])
+def test_pair_list_without_cells_far_site(site):
+    s = systems.lj_fluid(ncell=7, seed=4, jitter_star=0.1)
+    s.config.use_cell_list = False
+    ens = engine.GpuEnsemble(s, precision="mixed")
+    pos = s.pos.copy()
+    pos[site, 0] += 10 * ens.box
+    ens.upload_positions(pos)
+    p = ens.pairs()
+    assert not (p == site).any()
+    f, _, _ = ens.compute_forces()
+    assert not f[site].any()
+    # pair forces of 1e3 to 1e4 kJ/mol/nm, each side in FP32: 1e-7 of that a pair
+    assert np.abs(f.sum(0)).max() < 1e-2
+    ens.close()
