@@ -251,11 +251,12 @@ __device__ __forceinline__ void shake_mol(const IntArgs &a, int m, int s, int ns
                 double nx_ = rn[i][0] - rn[nx][0], ny_ = rn[i][1] - rn[nx][1], nz_ = rn[i][2] - rn[nx][2];
                 if (decltype(pbc)::value) pbc3(nx_, ny_, nz_, a.box);
                 const double diff = len2[i] - (nx_ * nx_ + ny_ * ny_ + nz_ * nz_);
-                const bool need = fabs(diff) > len2[i] * tol2;
+                const bool off = fabs(diff) > len2[i] * tol2;
                 const double ox = ob[i][0], oy = ob[i][1], oz = ob[i][2];
                 const double rr = ox * nx_ + oy * ny_ + oz * nz_;
-                geom = geom || (need && rr < len2[i] * a.shake_tol);
-                done = done && !need;
+                geom = geom || (off && rr < len2[i] * a.shake_tol);
+                const bool need = off && !geom;   // from a failure on nothing moves
+                done = done && !off;
                 const double B = rr * (2 * (mr[i] + mr[nx]));
                 double e = fma(-B, y[i], 1.0);
                 if (need && !(fabs(e) <= 0x1p-7)) {

@@ -117,3 +117,34 @@ def test_list_overflow():
     f1, _, _ = ens.compute_forces()
     assert rms_rel(f1, f0) < 1e-12
     ens.close()
+
+
+def test_shake_geometric_failure():
+    """A bond whose new vector is not along its old one fails as SHAKE's
+    geometric failure, the sites left where the free step put them: two sites
+    meet in one step (no forces, so the product of old and new bond is 0)."""
+    s = systems.spce_water(nmol=27, box=2.4, cutoff=0.7, kmax=5, seed=2)
+    s.config.compute_ewald = False
+    s.config.timestep = 2.0 ** -10
+    for t in s.atom_types:
+        t.charge = t.eps = 0.0
+    pos = s.pos.copy()
+    pos[:3] = [[0.125, 0, 0], [0, 0, 0], [0, 0.1, 0]]
+    vel = np.zeros((s.n_atoms, 3))
+    vel[0, 0] = -128.0
+    vel[4, 0] = 128.0 * s.masses()[0] / s.masses()[4]   # no net momentum
+    ens = engine.GpuEnsemble(s, velocities=vel)
+    ens.upload_positions(pos)
+    lf = engine.LFIntegrator(ens)
+    lf.start()
+    code, msg = _status(lambda: lf.run(1))
+    assert code == L.SMD_ERR_SHAKE and "geometric" in msg, msg
+    st = ens.state()
+    assert np.array_equal(st["pos"][:3], [[0, 0, 0], [0, 0, 0], [0, 0.1, 0]])
+    assert all(np.isfinite(x).all() for x in st.values())
+    # the context stays usable
+    ens.upload_positions(s.pos)
+    ens.upload_velocities(np.zeros_like(vel))
+    lf.start()
+    lf.run(1)
+    ens.close()
