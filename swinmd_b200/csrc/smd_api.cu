@@ -960,7 +960,7 @@ int smd_set_wait_limit(smd_ctx *x, double seconds) {
 }
 
 int smd_test_skip_arrival(smd_ctx *x, int block) {
-    if (!x || block < -1 || (block >= 0 && block >= x->c.cg_blocks))
+    if (!x || block < -1 || (block >= 0 && block >= solve_grid(x->c)))
         return fail(x, SMD_ERR_ARG, "smd_test_skip_arrival: block must be -1 or a block of the dipole solve");
     x->c.test_skip_block = block;
     x->c.graph_dirty = 1;

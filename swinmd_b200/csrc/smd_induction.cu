@@ -2137,7 +2137,6 @@ int setup_cg(Ctx &c) {
         for (const void *k : ps)
             if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room) != cudaSuccess)
                 return SMD_ERR_CUDA;
-        
     }
     return 0;
 }
@@ -2256,6 +2255,29 @@ void launch_blk_response(Ctx &c, double *out, int order, double *out_prev) {
 
 // the PCG solve from the start dipoles, then the site records' new dipoles
 // and the step's dipole history
+// the solve has inverse molecule blocks (built by launch_ind_field)
+static bool solve_blocks(const Ctx &c) { return c.cg_precond == SMD_PRECOND_MOLECULE && c.cg_blk; }
+
+// The pipelined form, and within it the one with the vector in shared memory.
+// The pipelined recurrences drift by rounding, which limits the change they
+// can resolve: tight tolerances (the checkers' 1e-13) keep the
+// single-reduction form.  Mode 1 (the default): the mixed path only; in FP64
+// the single-reduction form is the faster one (double4 gathers; 0.450 against
+// 0.480 ms for 4096 molecules); mode 2: both precisions.
+static bool solve_pipelined(const Ctx &c) {
+    return solve_blocks(c) && c.pp_blocks > 0 && c.cg_pipelined >= (c.precision == SMD_PREC_MIXED ? 1 : 2) &&
+           c.cg_tol >= PP_MIN_TOL;
+}
+static PcgShape solve_shared(const Ctx &c) {
+    if (c.precision != SMD_PREC_MIXED || !solve_pipelined(c)) return PcgShape{};
+    return pcg_shared_shape(c.nmol, c.ind_cap, c.ps_sms, c.ps_smem);
+}
+
+int solve_grid(const Ctx &c) {
+    const PcgShape s = solve_shared(c);
+    return s.threads > 0 ? s.blocks : (solve_pipelined(c) ? c.pp_blocks : c.cg_blocks);
+}
+
 void launch_ind_cg(Ctx &c) {
     IndArgs a = ind_args(c);
     const bool f32 = c.precision == SMD_PREC_MIXED;
@@ -2272,10 +2294,10 @@ void launch_ind_cg(Ctx &c) {
     g.part = c.cgs + CG_SCAL + CG_TRACE; g.scal = c.cgs; g.bar = c.cg_bar; g.status = c.status;
     g.wait_ns = c.wait_ns;
     g.skip_block = c.test_skip_block;
-    g.nblocks = c.cg_blocks; g.max_iter = c.cg_max_iter; g.tol = c.cg_tol;
+    g.nblocks = solve_grid(c); g.max_iter = c.cg_max_iter; g.tol = c.cg_tol;
     // 0: start from alpha E0; 1: start from the dipoles in p (previous solve or network)
     g.guess = (c.cg_guess == SMD_GUESS_PREVIOUS || guess_order(c) > 0 || learned) ? 1 : 0;
-    const bool bj = c.cg_precond == SMD_PRECOND_MOLECULE && c.cg_blk;   // blocks built by launch_ind_field
+    const bool bj = solve_blocks(c);
     g.blk = c.cg_blk;
     // the mixed path's site records take the dipoles inside the solve
     g.srec = f32 && c.srec ? (float *)c.srec : nullptr;
@@ -2283,7 +2305,7 @@ void launch_ind_cg(Ctx &c) {
     // cooperative launch: the runtime refuses it unless every block can be
     // resident at once, which the grid barrier relies on
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(c.cg_blocks);
+    cfg.gridDim = dim3(g.nblocks);
     cfg.blockDim = dim3(CG_THREADS);
     cfg.stream = c.stream;
     cudaLaunchAttribute attr[1];
@@ -2292,24 +2314,14 @@ void launch_ind_cg(Ctx &c) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     g.w = c.cgw + 26 * n; g.m = c.cgw + 29 * n; g.q = c.cgw + 32 * n;
-    // the pipelined recurrences drift by rounding, which limits the change
-    // they can resolve: tight tolerances (the checkers' 1e-13) keep the
-    // single-reduction form
-    // mode 1 (the default): the mixed path only; in FP64 the single-reduction
-    // form is the faster one (double4 gathers; 0.450 against 0.480 ms on
-    // polwater4096); mode 2: both precisions
-    if (bj && c.pp_blocks > 0 && c.cg_pipelined >= (f32 ? 1 : 2) && c.cg_tol >= PP_MIN_TOL) {
-        g.nblocks = c.pp_blocks;
-        cfg.gridDim = dim3(c.pp_blocks);
+    if (solve_pipelined(c)) {
         cfg.blockDim = dim3(PP_THREADS);
-        const PcgShape s = pcg_shared_shape(c.nmol, c.ind_cap, c.ps_sms, c.ps_smem);
-        if (f32 && s.threads > 0) {
+        const PcgShape s = solve_shared(c);
+        if (s.threads > 0) {
             PcgShared h;
             h.mols = s.mols; h.slots = s.slots;
             h.vec = (float *)g.g0;
             h.nv = (c.n + 3) & ~3;
-            g.nblocks = s.blocks;
-            cfg.gridDim = dim3(s.blocks);
             cfg.blockDim = dim3(s.threads);
             cfg.dynamicSmemBytes = s.smem;
             with_lanes(s.tpp, [&](auto l) { cudaLaunchKernelEx(&cfg, k_ind_pcg_shared<decltype(l)::value>, g, h); });

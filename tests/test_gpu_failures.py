@@ -148,3 +148,23 @@ def test_shake_geometric_failure():
     lf.start()
     lf.run(1)
     ens.close()
+
+
+@pytest.mark.parametrize("precision,nmol", [("fp64", 216), ("mixed", 1331), ("mixed", 4096)])
+def test_skip_arrival_takes_the_solve_s_blocks(precision, nmol):
+    """The hook takes the blocks of the solve that the settings choose and no
+    others: the last one it takes is missed at the barrier."""
+    ens = engine.GpuEnsemble(systems.polarizable_water(nmol=nmol, kmax=7, seed=3), precision=precision)
+    skip = lambda b: ens._chk(ens.lib.smd_test_skip_arrival(ens.ctx, b))   # noqa: E731
+    lo, hi = 0, 1 << 20
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        lo, hi = (mid, hi) if _status(lambda: skip(mid))[0] == L.SMD_OK else (lo, mid)
+    ens._chk(ens.lib.smd_set_wait_limit(ens.ctx, 1e-3))
+    skip(lo)
+    code, msg = _status(lambda: ens.compute_forces(L.TERM_IND_SHORT))
+    assert code == L.SMD_ERR_TIMEOUT, msg
+    skip(-1)
+    ens._chk(ens.lib.smd_set_wait_limit(ens.ctx, 1.0))
+    ens.compute_forces(L.TERM_IND_SHORT)
+    ens.close()
