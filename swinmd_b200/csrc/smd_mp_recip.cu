@@ -873,13 +873,17 @@ __device__ __forceinline__ double2 pfma(double2 a, double2 b, double2 c) {
     return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
 }
 
+// holds a value's uses behind the stores written before it
+__device__ __forceinline__ void pin(float &x) { asm volatile("" : "+f"(x) : : "memory"); }
+__device__ __forceinline__ void pin(double &x) { asm volatile("" : "+d"(x) : : "memory"); }
+
 // item[b * CS_ITEMS + t] = (column within the block's group, nz range) or
 // (-1, 0); grp[b] = (first column, columns)
 template <typename T, bool IND>
 __global__ void __launch_bounds__(CS_ITEMS, 3) k_col_sums(int n, int chunk, int nt, int row, double vx, double vy, double vz,
                                                        const int2 *grp, const int2 *item, const int4 *col,
                                                        const typename ColT<T>::T2 *stab,
-                                                       const typename ColT<T>::T4 *ssv, T *part) {
+                                                       const typename ColT<T>::T4 *ssv, double *part) {
     using T2 = typename ColT<T>::T2;
     using T4 = typename ColT<T>::T4;
     constexpr int NZ = ColP<T>::NZ, NU = IND ? 5 : 3;
@@ -990,19 +994,26 @@ __global__ void __launch_bounds__(CS_ITEMS, 3) k_col_sums(int n, int chunk, int 
     __pipeline_wait_prior(0);
     if (!own) return;
     // F and G at +kz and -kz: U = U0 + kz U1 (+ kz^2 U2), S(+) = al + i be,
-    // S(-) = al' - i be' with the odd powers of kz negated
+    // S(-) = al' - i be' with the odd powers of kz negated; FP64 from here on
     const size_t ns = (size_t)gridDim.x * CS_ITEMS, me = blockIdx.x * CS_ITEMS + threadIdx.x;
 #pragma unroll
     for (int j = 0; j < NZ; j++) {
-        const T kz = (T)((it.y * NZ + j) * vz), k2 = kz * kz;
-        T *o = part + ((size_t)blockIdx.y * NZ + j) * 8 * ns + me;
+        const double kz = (it.y * NZ + j) * vz, k2 = kz * kz;
+#pragma unroll
+        for (int k = 0; k < NU; k++)   // one nz's conversions after the last one's stores: all at once spill
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                pin(acc[j][k][q].x);
+                pin(acc[j][k][q].y);
+            }
+        double *o = part + ((size_t)blockIdx.y * NZ + j) * 8 * ns + me;
 #pragma unroll
         for (int f = 0; f < (IND ? 2 : 1); f++) {
-            T ev[4], od[4];   // Re, Im of sum U Re Z, Re, Im of sum U Im Z
+            double ev[4], od[4];   // Re, Im of sum U Re Z, Re, Im of sum U Im Z
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                auto at = [&](int k) { return q & 1 ? acc[j][k][q >> 1].y : acc[j][k][q >> 1].x; };
-                ev[q] = f == 0 ? tfma(k2, at(2), at(0)) : at(IND ? 3 : 0);
+                auto at = [&](int k) { return (double)(q & 1 ? acc[j][k][q >> 1].y : acc[j][k][q >> 1].x); };
+                ev[q] = f == 0 ? fma(k2, at(2), at(0)) : at(IND ? 3 : 0);
                 od[q] = kz * (f == 0 ? at(1) : at(IND ? 4 : 0));
             }
             o[(4 * f + 0) * ns] = (ev[0] + od[0]) - (ev[3] + od[3]);
@@ -1018,7 +1029,7 @@ __global__ void __launch_bounds__(CS_ITEMS, 3) k_col_sums(int n, int chunk, int 
 template <typename T, bool IND>
 __global__ void __launch_bounds__(32 * CR_ROWS, 2) k_col_reduce(int nblk, int chunks, int zn, double vx, double vy,
                                                              double vz, double pi4V, double aR4, const int2 *grp,
-                                                             const int2 *item, const int4 *col, const T *part,
+                                                             const int2 *item, const int4 *col, const double *part,
                                                              typename ColT<T>::T4 *coef, double *tot) {
     constexpr int NZ = ColP<T>::NZ, NV = IND ? 8 : 4;
     __shared__ double s_p[CR_ROWS][NV][32];
@@ -1035,9 +1046,9 @@ __global__ void __launch_bounds__(32 * CR_ROWS, 2) k_col_reduce(int nblk, int ch
     double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (nz <= cc.z)
         for (int ch = ty; ch < chunks; ch += CR_ROWS) {
-            const T *o = part + ((size_t)ch * NZ + j) * 8 * ns + me;
+            const double *o = part + ((size_t)ch * NZ + j) * 8 * ns + me;
 #pragma unroll
-            for (int q = 0; q < NV; q++) v[q] += (double)o[q * ns];
+            for (int q = 0; q < NV; q++) v[q] += o[q * ns];
         }
 #pragma unroll
     for (int q = 0; q < NV; q++) s_p[ty][q][tx] = v[q];
@@ -1364,8 +1375,8 @@ int mp_recip_prepare(Ctx &c) {
         const int chunk = col_chunk(c.n, R.mblk[q], sm_count() * blocks_per_sm(kern, CS_ITEMS, sm));
         R.mchunk[q] = chunk;
         const size_t sz = q == 0 ? sizeof(float) : sizeof(double);
-        part = std::max(part, sz * (size_t)((c.n + chunk - 1) / chunk) * NZ * 8 * item.size() +
-                                  sizeof(double) * 8 * (item.size() / 32) * NZ);
+        part = std::max(part, sizeof(double) * 8 * NZ *
+                                  ((size_t)((c.n + chunk - 1) / chunk) * item.size() + item.size() / 32));
         // zeroed: the force pass reads entries past a column's end, which the
         // reduction never writes
         const size_t coef = 4 * sz * mcol.size() * (q == 0 ? col_zn<float>(nt - 1) : col_zn<double>(nt - 1));
@@ -1489,7 +1500,7 @@ void column_terms(Ctx &c, int slot_e, int slot_e2) {
     column_tables<T>(c, stab, ssv);
     const int rb = nblk * (CS_ITEMS / 32);
     double *tot = (double *)R.mpart;   // the blocks' energies and virial, ahead of the partial sums
-    T *part = (T *)(tot + 8 * (size_t)rb * NZ);
+    double *part = tot + 8 * (size_t)rb * NZ;
     k_col_sums<T, IND><<<dim3(nblk, chunks), CS_ITEMS, col_sums_smem<T>(R.row, IND), c.stream>>>(
         c.n, chunk, nt, R.row, vx, vy, vz, R.mgrp[q], R.mitem[q], R.mcol, stab, ssv, part);
     k_col_reduce<T, IND><<<dim3(rb, NZ), 32 * CR_ROWS, 0, c.stream>>>(
