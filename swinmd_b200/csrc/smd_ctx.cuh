@@ -74,11 +74,11 @@ struct Recip {               // Ewald reciprocal space (k half-space, k^2 < kcut
     int nseg = 0, ncol = 0, row = 0, tab_n = 0;
     int4 *kseg = nullptr;    // runs of <= 4 k of one column (first k, count, nx | ny << 16, first nz)
     int4 *mcol = nullptr;    // columns (nx, ny, largest nz, 0)
-    // column products, FP32 [0] and FP64 [1]: blocks, sites per block, their
-    // column groups (first, count) and (column, nz range) items
-    int mblk[2] = {0, 0}, mchunk[2] = {0, 0};
+    // column products, FP32 [0] and FP64 [1]: column groups, sites per chunk,
+    // rows of blocks, the groups (first, count) and their (column, nz range) items
+    int mblk[2] = {0, 0}, mchunk[2] = {0, 0}, mrows[2] = {0, 0};
     int2 *mgrp[2] = {nullptr, nullptr}, *mitem[2] = {nullptr, nullptr};
-    void *mpart = nullptr;   // block totals [blocks][8], partial sums [chunks][nz][8][items]
+    void *mpart = nullptr;   // block totals [blocks][8], partial sums [rows][nz][8][items]
     void *mcoef[2] = {nullptr, nullptr};   // force coefficients [ncol][nz] of 4, FP32 and FP64
     float2 *stab = nullptr;  // per site phase tables [n][row]: e^{2 pi i m f / 2^32}, m < nmax + 1, per axis
     // the FP64 column passes: phase tables e^{2 pi i m f / 2^64} and FP64 site

@@ -836,7 +836,9 @@ __device__ __forceinline__ void add_moments(int n, int i, const double4 *pos4, c
 // threads first form the five numbers of every (site, column) of a sub-tile
 // in shared memory, then each accumulates CS_NZ nz of one column over the
 // sub-tile (the same numbers serve all its nz ranges).  Running sums are T
-// within a chunk of at most 128 sites, FP64 across chunks (k_col_reduce).
+// within a chunk of at most 128 sites, FP64 across chunks: the launches of later
+// slabs of sites add to the first one's sums in memory, k_col_reduce adds the
+// blocks'.  (A loop over chunks in the kernel: 200 -> 207 us.)
 //
 // k_col_force: one thread per site, Z^nz in registers.  With conj H = B + iA
 // times e^{-ia} folded over +-nz (E = conj H+ + conj H-, D = conj H+ - conj
@@ -880,7 +882,7 @@ __device__ __forceinline__ void pin(double &x) { asm volatile("" : "+d"(x) : : "
 // item[b * CS_ITEMS + t] = (column within the block's group, nz range) or
 // (-1, 0); grp[b] = (first column, columns)
 template <typename T, bool IND>
-__global__ void __launch_bounds__(CS_ITEMS, 3) k_col_sums(int n, int chunk, int nt, int row, double vx, double vy, double vz,
+__global__ void __launch_bounds__(CS_ITEMS, 3) k_col_sums(int n, int slab, int chunk, int nt, int row, double vx, double vy, double vz,
                                                        const int2 *grp, const int2 *item, const int4 *col,
                                                        const typename ColT<T>::T2 *stab,
                                                        const typename ColT<T>::T4 *ssv, double *part) {
@@ -895,7 +897,8 @@ __global__ void __launch_bounds__(CS_ITEMS, 3) k_col_sums(int n, int chunk, int 
     __shared__ int s_o[2][CS_COLS];                      // the column's X and Y entries (Y negated: conjugate)
     const int2 g = grp[blockIdx.x], it = item[blockIdx.x * CS_ITEMS + threadIdx.x];
     const bool own = it.x >= 0;
-    const int s0 = blockIdx.y * chunk, s1 = min(n, s0 + chunk);
+    const int s0 = (slab * gridDim.y + blockIdx.y) * chunk, s1 = min(n, s0 + chunk);
+    if (s0 >= n) return;   // a short last slab
     const int srow = row | 1, tstride = CS_SUB * srow + CS_PAD;
     for (int e = threadIdx.x; e < g.y; e += CS_ITEMS) {
         const int4 cc = col[g.x + e];
@@ -1016,18 +1019,22 @@ __global__ void __launch_bounds__(CS_ITEMS, 3) k_col_sums(int n, int chunk, int 
                 ev[q] = f == 0 ? fma(k2, at(2), at(0)) : at(IND ? 3 : 0);
                 od[q] = kz * (f == 0 ? at(1) : at(IND ? 4 : 0));
             }
-            o[(4 * f + 0) * ns] = (ev[0] + od[0]) - (ev[3] + od[3]);
-            o[(4 * f + 1) * ns] = (ev[1] + od[1]) + (ev[2] + od[2]);
-            o[(4 * f + 2) * ns] = (ev[0] - od[0]) + (ev[3] - od[3]);
-            o[(4 * f + 3) * ns] = (ev[1] - od[1]) - (ev[2] - od[2]);
+            const double v[4] = {(ev[0] + od[0]) - (ev[3] + od[3]), (ev[1] + od[1]) + (ev[2] + od[2]),
+                                 (ev[0] - od[0]) + (ev[3] - od[3]), (ev[1] - od[1]) - (ev[2] - od[2])};
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                double *at = o + (4 * f + q) * ns;
+                if (slab > 0) atomicAdd(at, v[q]);   // this thread's alone: a load would be waited for
+                else *at = v[q];
+            }
         }
     }
 }
 
-// F(+-k), G(+-k) in fixed chunk order for 32 items at one nz of each:
+// F(+-k), G(+-k) in fixed order of the rows for 32 items at one nz of each:
 // energies, long virial and the force pass's coefficients 2c (E, D)
 template <typename T, bool IND>
-__global__ void __launch_bounds__(32 * CR_ROWS, 2) k_col_reduce(int nblk, int chunks, int zn, double vx, double vy,
+__global__ void __launch_bounds__(32 * CR_ROWS, 2) k_col_reduce(int nblk, int rows, int zn, double vx, double vy,
                                                              double vz, double pi4V, double aR4, const int2 *grp,
                                                              const int2 *item, const int4 *col, const double *part,
                                                              typename ColT<T>::T4 *coef, double *tot) {
@@ -1045,7 +1052,7 @@ __global__ void __launch_bounds__(32 * CR_ROWS, 2) k_col_reduce(int nblk, int ch
     const int nz = it.y * NZ + j;
     double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (nz <= cc.z)
-        for (int ch = ty; ch < chunks; ch += CR_ROWS) {
+        for (int ch = ty; ch < rows; ch += CR_ROWS) {
             const double *o = part + ((size_t)ch * NZ + j) * 8 * ns + me;
 #pragma unroll
             for (int q = 0; q < NV; q++) v[q] += o[q * ns];
@@ -1286,6 +1293,15 @@ int col_chunk(int n, int nblk, int resident) {
     return best;
 }
 
+// rows of blocks of a launch of the sums pass, one chunk each, whose sums take
+// at most 512 MB (one row if that is more).  One launch needs 1.1 GB at 60 000
+// sites and |n| < 32 and grows with the sites
+int col_rows(int chunks, size_t row_bytes) {
+    const int most = (int)std::max<size_t>(1, ((size_t)512 << 20) / row_bytes);
+    const int launches = (chunks + most - 1) / most;
+    return (chunks + launches - 1) / launches;
+}
+
 // column, run and item records of the column passes, the site-table and
 // site-record buffers of both precisions and the kernels' dynamic shared
 // memory (once per k set, outside any capture).  Leaves the column passes
@@ -1300,7 +1316,7 @@ int mp_recip_prepare(Ctx &c) {
         if (p) cudaFree(p);
     R.kseg = nullptr; R.mcol = nullptr; R.stab = nullptr; R.stab_d = nullptr; R.srec_d = nullptr;
     R.mpart = nullptr;
-    for (int q = 0; q < 2; q++) { R.mcoef[q] = nullptr; R.mgrp[q] = nullptr; R.mitem[q] = nullptr; R.mblk[q] = R.mchunk[q] = 0; }
+    for (int q = 0; q < 2; q++) { R.mcoef[q] = nullptr; R.mgrp[q] = nullptr; R.mitem[q] = nullptr; R.mblk[q] = R.mchunk[q] = R.mrows[q] = 0; }
     R.nseg = R.ncol = R.row = 0;
     if (nk == 0 || c.n == 0 || c.rc.nmax + 1 > TAB_MAX || !c.srec) return 0;
     std::vector<int> kn(3 * (size_t)nk);
@@ -1373,10 +1389,11 @@ int mp_recip_prepare(Ctx &c) {
         const void *kern = q == 0 ? (const void *)k_col_sums<float, true> : (const void *)k_col_sums<double, true>;
         const size_t sm = q == 0 ? col_sums_smem<float>(row, true) : col_sums_smem<double>(row, true);
         const int chunk = col_chunk(c.n, R.mblk[q], sm_count() * blocks_per_sm(kern, CS_ITEMS, sm));
+        const size_t bytes = sizeof(double) * 8 * NZ * item.size();   // of a row of partial sums
         R.mchunk[q] = chunk;
+        R.mrows[q] = col_rows((c.n + chunk - 1) / chunk, bytes);
+        part = std::max(part, bytes * R.mrows[q] + bytes / 32);       // and the blocks' totals
         const size_t sz = q == 0 ? sizeof(float) : sizeof(double);
-        part = std::max(part, sizeof(double) * 8 * NZ *
-                                  ((size_t)((c.n + chunk - 1) / chunk) * item.size() + item.size() / 32));
         // zeroed: the force pass reads entries past a column's end, which the
         // reduction never writes
         const size_t coef = 4 * sz * mcol.size() * (q == 0 ? col_zn<float>(nt - 1) : col_zn<double>(nt - 1));
@@ -1492,7 +1509,7 @@ void column_terms(Ctx &c, int slot_e, int slot_e2) {
     constexpr int q = sizeof(T) == 4 ? 0 : 1, NZ = ColP<T>::NZ;
     const Recip &R = c.rc;
     const int nt = R.nmax + 1, zn = col_zn<T>(R.nmax), nblk = R.mblk[q];
-    const int chunk = R.mchunk[q], chunks = (c.n + chunk - 1) / chunk;
+    const int chunk = R.mchunk[q], rows = R.mrows[q];
     const double PI2 = 6.283185307179586476925, vx = PI2 / c.box.L[0], vy = PI2 / c.box.L[1], vz = PI2 / c.box.L[2];
     const double vol = c.box.L[0] * c.box.L[1] * c.box.L[2];
     T2 *stab;
@@ -1501,10 +1518,11 @@ void column_terms(Ctx &c, int slot_e, int slot_e2) {
     const int rb = nblk * (CS_ITEMS / 32);
     double *tot = (double *)R.mpart;   // the blocks' energies and virial, ahead of the partial sums
     double *part = tot + 8 * (size_t)rb * NZ;
-    k_col_sums<T, IND><<<dim3(nblk, chunks), CS_ITEMS, col_sums_smem<T>(R.row, IND), c.stream>>>(
-        c.n, chunk, nt, R.row, vx, vy, vz, R.mgrp[q], R.mitem[q], R.mcol, stab, ssv, part);
+    for (int slab = 0; (long long)slab * rows * chunk < c.n; slab++)
+        k_col_sums<T, IND><<<dim3(nblk, rows), CS_ITEMS, col_sums_smem<T>(R.row, IND), c.stream>>>(
+            c.n, slab, chunk, nt, R.row, vx, vy, vz, R.mgrp[q], R.mitem[q], R.mcol, stab, ssv, part);
     k_col_reduce<T, IND><<<dim3(rb, NZ), 32 * CR_ROWS, 0, c.stream>>>(
-        nblk, chunks, zn, vx, vy, vz, 2.0 * PI2 * (1.0 / vol), 1.0 / (4.0 * c.ew_alpha * c.ew_alpha), R.mgrp[q],
+        nblk, rows, zn, vx, vy, vz, 2.0 * PI2 * (1.0 / vol), 1.0 / (4.0 * c.ew_alpha * c.ew_alpha), R.mgrp[q],
         R.mitem[q], R.mcol, part, (T4 *)R.mcoef[q], tot);
     // column ranges of the force pass: about one wave of blocks, at least
     // eight columns each (a range starts with a sine and cosine)

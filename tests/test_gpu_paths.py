@@ -187,3 +187,33 @@ def test_pair_list_without_cells_far_site(site):
     # pair forces of 1e3 to 1e4 kJ/mol/nm, each side in FP32: 1e-7 of that a pair
     assert np.abs(f.sum(0)).max() < 1e-2
     ens.close()
+
+
+# the column products' workspace: at most 512 MB of partial sums, the site
+# tables (96 entries of 8 and of 16 bytes and a record of 128 bytes a site) and
+# coefficients and items below 32 MB; the k set past the tables (kmax 33) takes
+# none of it.  Past that size the sums go in several launches
+def test_multipole_columns_workspace():
+    import torch
+    free = lambda: torch.cuda.mem_get_info()[0]   # noqa: E731
+    s = systems.polarizable_water(nmol=20000, cutoff=0.9, switch=0.8, kmax=32, seed=7)
+    n, k32 = s.n_atoms, s.config.k_cutoff
+    torch.zeros(1, device="cuda")
+    used = []
+    for kcut in (k32 * np.sqrt((33 ** 2 - 0.5) / (32 ** 2 - 0.5)), k32):
+        s.config.k_cutoff = kcut
+        before = free()
+        ens = engine.GpuEnsemble(s)
+        used.append(before - free())
+        if kcut > k32:
+            ens.close()
+    assert used[1] - used[0] < (512 << 20) + n * (96 * 24 + 128) + (32 << 20)
+    ens.set_reference_forms(True)
+    fr, er, _ = ens.compute_forces(L.TERM_MP_LONG)
+    ens.set_reference_forms(False)
+    for precision, tol in (("fp64", 1e-10), ("mixed", 1e-6)):
+        ens.set_precision(precision)
+        f, e, _ = ens.compute_forces(L.TERM_MP_LONG)
+        assert rms_rel(f, fr) < tol
+        assert abs(e[L.E_LONG] - er[L.E_LONG]) <= tol * abs(er[L.E_LONG])
+    ens.close()
