@@ -22,8 +22,9 @@
 // sites and 900 k).
 //
 // Three kernels: partial sums over (column item x site chunk) blocks, a
-// fixed-order reduction over chunks that also forms the energy, the virial
-// and the force coefficients, and a per-site force pass.
+// fixed-order reduction over chunks that also forms the force coefficients and
+// the blocks' energies and virial, and a per-site force pass, one more block of
+// which adds those up.
 //
 // Sheared cell (SLLOD with Lees-Edwards images; no reference code): the
 // images of the box with offset d form the lattice a1 = (Lx, 0, 0),
@@ -214,16 +215,17 @@ __global__ void __launch_bounds__(ES_THREADS) k_ew_sums(EwArgs a, double *part) 
     }
 }
 
-// S(+-k) in fixed chunk order for 32 columns at one nz: energy, long virial
-// and the force coefficients 2c (conj S+ + conj S-), 2c (conj S+ - conj S-)
-// (zero for an nz the column does not hold)
-constexpr int ER_ROWS = 8;
+// S(+-k) in fixed chunk order for 32 columns at one nz: energy and long virial
+// (tot[nz][block of columns][8]: E, xx, yy, zz, xy, xz, yz, 0) and the force
+// coefficients 2c (conj S+ + conj S-), 2c (conj S+ - conj S-) (zero for an nz
+// the column does not hold)
+constexpr int ER_ROWS = 8, ER_COLS = 32;
 __global__ void __launch_bounds__(32 * ER_ROWS) k_ew_reduce(EwArgs a, int nzp, int nzt, int chunks, const double *part,
-                                                            double4 *coef, long long *acc) {
+                                                            double4 *coef, double *tot) {
     __shared__ double s_p[ER_ROWS][4][32];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int ncol = *a.ncol, ci = blockIdx.x * 32 + tx, nz = blockIdx.y;
-    if ((int)blockIdx.x * 32 >= ncol) return;   // block-uniform
+    const int ncol = *a.ncol, ci = blockIdx.x * ER_COLS + tx, nz = blockIdx.y;
+    if ((int)blockIdx.x * ER_COLS >= ncol) return;   // block-uniform
     const int4 cc = ci < ncol ? a.col[ci] : make_int4(0, 0, -1, 0);
     const bool live = cc.z >= nz / nzt * nzt;   // the sums pass wrote this slot
     double v[4] = {0, 0, 0, 0};
@@ -270,18 +272,33 @@ __global__ void __launch_bounds__(32 * ER_ROWS) k_ew_reduce(EwArgs a, int nzp, i
     e = warp_sum(e);
 #pragma unroll
     for (int q = 0; q < 6; q++) w[q] = warp_sum(w[q]);
-    if (tx < 7) {
-        double x = e;
+    if (tx < 8) {
+        double x = tx == 0 ? e : 0.0;
 #pragma unroll
         for (int q = 0; q < 6; q++)
             if (tx == q + 1) x = w[q];
-        const int slots[7][2] = {{ACC_E_LONG, -1},       {ACC_LVIR + 0, -1},       {ACC_LVIR + 4, -1},
-                                 {ACC_LVIR + 8, -1},     {ACC_LVIR + 1, ACC_LVIR + 3},
-                                 {ACC_LVIR + 2, ACC_LVIR + 6}, {ACC_LVIR + 5, ACC_LVIR + 7}};
-        const unsigned long long fx = (unsigned long long)to_fix(x, ACC_SCALE);
-        atomicAdd((unsigned long long *)&acc[slots[tx][0]], fx);
-        if (slots[tx][1] >= 0) atomicAdd((unsigned long long *)&acc[slots[tx][1]], fx);
+        tot[8 * ((size_t)nz * gridDim.x + blockIdx.x) + tx] = x;
     }
+}
+
+// The energy and the long virial from the live blocks' totals (nb of gx per
+// nz) in a fixed order, each rounded to fixed point once; one block
+__device__ __forceinline__ void ew_totals(int nzp, int gx, int nb, const double *tot, long long *acc,
+                                          double (*s)[8]) {
+    const int q = threadIdx.x & 7, row = threadIdx.x >> 3;
+    double x = 0;
+#pragma unroll 8
+    for (int b = row; b < nb * nzp; b += EF_THREADS / 8) x += tot[8 * ((size_t)(b / nb) * gx + b % nb) + q];
+    s[row][q] = x;
+    __syncthreads();
+    if (threadIdx.x >= 7) return;
+    for (int r = 1; r < EF_THREADS / 8; r++) x += s[r][q];
+    const int slots[7][2] = {{ACC_E_LONG, -1},       {ACC_LVIR + 0, -1},       {ACC_LVIR + 4, -1},
+                             {ACC_LVIR + 8, -1},     {ACC_LVIR + 1, ACC_LVIR + 3},
+                             {ACC_LVIR + 2, ACC_LVIR + 6}, {ACC_LVIR + 5, ACC_LVIR + 7}};
+    const unsigned long long fx = (unsigned long long)to_fix(x, ACC_SCALE);
+    atomicAdd((unsigned long long *)&acc[slots[q][0]], fx);
+    if (slots[q][1] >= 0) atomicAdd((unsigned long long *)&acc[slots[q][1]], fx);
 }
 
 // Per-site force.  The blocks of a cluster (along y) split the columns, so
@@ -291,10 +308,11 @@ __global__ void __launch_bounds__(32 * ER_ROWS) k_ew_reduce(EwArgs a, int nzp, i
 // nz; the column's X^nx Y^ny follows from the one before along ny.  FP64
 // issue bounds it (8000 ions, 2094 k: 67 M FMAs, 4 us).
 template <int NZT>
-__global__ void __launch_bounds__(EF_THREADS) k_ew_force(EwArgs a, const double4 *coef, long long *frc) {
+__global__ void __launch_bounds__(EF_THREADS) k_ew_force(EwArgs a, const double4 *coef, long long *frc, const double *tot,
+                                                         long long *acc) {
     __shared__ double4 s_co[EF_COLS * NZT];
     __shared__ int4 s_col[EF_COLS];
-    __shared__ double s_f[3][EF_THREADS];
+    __shared__ double s_f[3][EF_THREADS], s_tot[EF_THREADS / 8][8];
     const int i = blockIdx.x * EF_THREADS + threadIdx.x;
     const bool own = i < a.n;
     const double dd = le_reduced(a.le, a.box);
@@ -302,6 +320,11 @@ __global__ void __launch_bounds__(EF_THREADS) k_ew_force(EwArgs a, const double4
     const double3 f = ew_frac(p, dd, a.box);
     const double2 z1 = ew_phase(f.z), y1 = ew_phase(f.y);
     const int ncol = *a.ncol, nzp = a.nch * NZT;
+    if (blockIdx.x == gridDim.x - 1) {   // past the sites; its whole cluster leaves here
+        if (blockIdx.y == 0)
+            ew_totals(nzp, (a.cap + ER_COLS - 1) / ER_COLS, (ncol + ER_COLS - 1) / ER_COLS, tot, acc, s_tot);
+        return;
+    }
     const int per = (ncol + gridDim.y - 1) / gridDim.y;
     const int c0 = blockIdx.y * per, c1 = min(ncol, c0 + per);
     double Fx = 0, Fy = 0, Fz = 0;
@@ -371,6 +394,11 @@ static int ew_nzt(int mmax) {
     return best;
 }
 
+// the reduction's totals, behind the partial sums
+static size_t ew_totals_size(const Recip &r) {
+    return (size_t)8 * r.ew_nch * r.ew_nzt * ((r.ew_cap + ER_COLS - 1) / ER_COLS);
+}
+
 // the column buffers: ncap columns with |nx| <= nxm, |ny| <= nym, nz <= mmax
 static int ew_alloc(Ctx &c, int ncap, int nxm, int nym, int mmax) {
     Recip &r = c.rc;
@@ -391,7 +419,7 @@ static int ew_alloc(Ctx &c, int ncap, int nxm, int nym, int mmax) {
     r.ew_chunks = std::max(1, std::min(sms, 2 * sms / std::max(gx, 1)));
     const size_t slots = (size_t)r.ew_nch * r.ew_nzt * ncap;
     if (!realloc(&r.ew_col, ncap) || !realloc(&r.ew_ncol, 1) || !realloc(&r.ew_coef, slots) ||
-        !realloc(&r.ew_part, slots * 4 * r.ew_chunks))
+        !realloc(&r.ew_part, slots * 4 * r.ew_chunks + ew_totals_size(r)))
         return SMD_ERR_CUDA;
     return cudaMemset(r.ew_ncol, 0, sizeof(int)) == cudaSuccess ? 0 : SMD_ERR_CUDA;
 }
@@ -511,15 +539,16 @@ static void launch_columns(Ctx &c, EwArgs a) {
     const int chunks = std::max(1, std::min(r.ew_chunks, (c.n + 7) / 8));
     const size_t smem = (size_t)a.tile * a.row * sizeof(double2);
     k_ew_sums<NZT><<<dim3((items + ES_THREADS - 1) / ES_THREADS, chunks), ES_THREADS, smem, c.stream>>>(a, r.ew_part);
-    k_ew_reduce<<<dim3((r.ew_cap + 31) / 32, nzp), 32 * ER_ROWS, 0, c.stream>>>(a, nzp, NZT, chunks, r.ew_part,
-                                                                               r.ew_coef, c.acc);
+    double *tot = r.ew_part + (size_t)nzp * r.ew_cap * 4 * r.ew_chunks;
+    k_ew_reduce<<<dim3((r.ew_cap + ER_COLS - 1) / ER_COLS, nzp), ER_COLS * ER_ROWS, 0, c.stream>>>(
+        a, nzp, NZT, chunks, r.ew_part, r.ew_coef, tot);
     // column ranges of the force pass (blocks of a cluster): about six blocks
     // per SM, at least four columns each
     const int nb = (c.n + EF_THREADS - 1) / EF_THREADS;
     int ranges = 8;
     while (ranges > 1 && (ranges * nb > 148 * 8 || ranges * 4 > r.ew_cap)) ranges /= 2;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nb, ranges);
+    cfg.gridDim = dim3(nb + 1, ranges);   // the last column of blocks: the totals
     cfg.blockDim = dim3(EF_THREADS);
     cfg.stream = c.stream;
     cudaLaunchAttribute attr[1];
@@ -529,7 +558,7 @@ static void launch_columns(Ctx &c, EwArgs a) {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_ew_force<NZT>, a, (const double4 *)r.ew_coef, c.frc);
+    cudaLaunchKernelEx(&cfg, k_ew_force<NZT>, a, (const double4 *)r.ew_coef, c.frc, (const double *)tot, c.acc);
 }
 
 void launch_recip(Ctx &c) {

@@ -217,3 +217,15 @@ def test_multipole_columns_workspace():
         assert rms_rel(f, fr) < tol
         assert abs(e[L.E_LONG] - er[L.E_LONG]) <= tol * abs(er[L.E_LONG])
     ens.close()
+
+
+# the point-charge reciprocal energy is rounded to its 2^-28 kJ/mol once; a few
+# FP64 roundings a term beside it
+@pytest.mark.parametrize("kmax", [9, 13, 17])
+def test_ewald_energy_rounding(kmax):
+    s = systems.nacl_melt(ncell=8, kmax=kmax, seed=2)
+    ens = engine.GpuEnsemble(s)
+    _, e, _ = ens.compute_forces(L.TERM_EWALD_LONG)
+    _, er, _ = _ewald_direct(s, ens.box, s.config.alpha, s.config.k_cutoff)
+    assert abs(e[L.E_LONG] - er) < 2.0 ** -29 + 1e-13 * abs(er)
+    ens.close()
