@@ -229,3 +229,38 @@ def test_ewald_energy_rounding(kmax):
     _, er, _ = _ewald_direct(s, ens.box, s.config.alpha, s.config.k_cutoff)
     assert abs(e[L.E_LONG] - er) < 2.0 ** -29 + 1e-13 * abs(er)
     ens.close()
+
+
+# either side of the lane rule's lines as they are (2600, 8000 and 12 000 sites),
+# against two lanes per site, which the rule never takes
+@pytest.mark.parametrize("kind,size,precision", [("lj", 8, "fp64"), ("lj", 9, "fp64"), ("lj", 12, "fp64"),
+                                                 ("lj", 13, "fp64"), ("lj", 14, "fp64"), ("lj", 15, "fp64"),
+                                                 ("lj", 14, "mixed"), ("lj", 15, "mixed"), ("spce", 866, "fp64"),
+                                                 ("spce", 867, "fp64"), ("spce", 866, "mixed"),
+                                                 ("spce", 867, "mixed")])
+def test_lanes_per_site_lines(kind, size, precision):
+    s = (systems.lj_fluid(ncell=size, seed=6, jitter_star=0.08) if kind == "lj" else
+         systems.spce_water(nmol=size, box=4.03 * (size / 2160) ** (1 / 3), seed=6, kmax=6))
+    f = []
+    for tpp in (0, 2):
+        ens = engine.GpuEnsemble(s, precision=precision, threads_per_site=tpp)
+        f.append(ens.compute_forces(L.TERM_VDW | L.TERM_EWALD_REAL)[0])
+        ens.close()
+    # sums of the same terms in another order, in units of 2^-32: FP64, and FP32
+    # of up to 280 terms a lane
+    assert rms_rel(f[0], f[1]) < (1e-11 if precision == "fp64" else 1e-6)
+
+
+# the polarisable kernels with 32 and with 16 lanes a site: mixed against FP64
+@pytest.mark.parametrize("nmol", [866, 867])
+def test_lanes_per_site_polarisable(nmol):
+    s = systems.polarizable_water(nmol=nmol, kmax=6, seed=5)
+    ens = engine.GpuEnsemble(s)
+    ens.set_solver(tol=1e-13, max_iter=1000)
+    f = []
+    for precision in ("fp64", "mixed"):
+        ens.set_precision(precision)
+        f.append([ens.compute_forces(t)[0] for t in (L.TERM_VDW, L.TERM_MP_SHORT, L.TERM_IND_SHORT, L.TERM_ALL)])
+    for a, b in zip(*f):
+        assert rms_rel(b, a) < 1e-6
+    ens.close()
