@@ -304,7 +304,11 @@ int smd_create(int device, smd_ctx **out) {
     if (!x) return SMD_ERR_ARG;
     Ctx &c = x->c;
     c.device = device;
-    if (cudaSetDevice(device) != cudaSuccess) { delete x; return SMD_ERR_CUDA; }
+    if (cudaSetDevice(device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        delete x;
+        return SMD_ERR_CUDA;
+    }
     if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess) {
         delete x;
         return SMD_ERR_CUDA;
@@ -887,7 +891,7 @@ int smd_set_multipole(smd_ctx *x, const double *type_mp, const double *polar, do
     CK(cudaMemset(c.e0, 0, 3 * n * sizeof(double)));
     int r = setup_cg(c);
     if (r) return fail(x, r, "smd_set_multipole: solver set-up failed");
-    const size_t cgb = (size_t)std::max(std::max(c.cg_blocks, c.pp_blocks), c.ps_sms);
+    const size_t cgb = (size_t)std::max(std::max(c.cg_blocks, c.pp_blocks), c.sms);
     CK(dalloc(&c.cgs, CG_SCAL + CG_TRACE + 16 * cgb));
     CK(cudaMemset(c.cgs, 0, (CG_SCAL + CG_TRACE + 16 * cgb) * sizeof(double)));
     CK(dalloc(&c.cg_bar, 2));

@@ -88,7 +88,7 @@ struct Recip {               // Ewald reciprocal space (k half-space, k^2 < kcut
 };
 
 struct Ctx {
-    int device = 0;
+    int device = 0, sms = 1;   // and its multiprocessors
     cudaStream_t stream = nullptr;
     std::string err;
     // sizes
@@ -150,8 +150,7 @@ struct Ctx {
     int cg_guess = 0;               // SMD_GUESS_*: 0 block solution of E0, 1 previous step, 2 learned, 3 first order
     int cg_blocks = 0;
     int pp_blocks = 0;              // grid of the pipelined solve (0: the layout does not allow it)
-    int ps_sms = 0;                 // the pipelined solve with the vector in shared memory: SMs (one block each)
-    size_t ps_smem = 0;             // and the shared memory a block may take
+    size_t ps_smem = 0;             // the pipelined solve with the vector in shared memory: what a block may take
     int cg_pipelined = 1;           // pipelined solve (molecule blocks): 0 never, 1 mixed path, 2 both precisions
     int cg_precond = SMD_PRECOND_MOLECULE;  // dipole-solve preconditioner
     double *cg_blk = nullptr;       // [nmol][81] inverse molecule blocks of A

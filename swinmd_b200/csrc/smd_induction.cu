@@ -2103,7 +2103,7 @@ int setup_cg(Ctx &c) {
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, c.device) != cudaSuccess) return SMD_ERR_CUDA;
     int want = (c.n * CG_TPP + CG_THREADS - 1) / CG_THREADS;
-    int maxb = per_sm * prop.multiProcessorCount;
+    int maxb = per_sm * c.sms;
     c.cg_blocks = want < maxb ? want : maxb;
     if (c.cg_blocks < 1) c.cg_blocks = 1;
     // the pipelined form: every molecule three sites, molecule k's at 3k .. 3k + 2
@@ -2121,10 +2121,9 @@ int setup_cg(Ctx &c) {
             return SMD_ERR_CUDA;
         v = v2 < v ? v2 : v;
         const int groups = (c.nmol + PP_MOLS - 1) / PP_MOLS;
-        const int mb = v * prop.multiProcessorCount;
+        const int mb = v * c.sms;
         c.pp_blocks = groups < mb ? groups : mb;
         // the form with the vector in shared memory: one block per SM
-        c.ps_sms = prop.multiProcessorCount;
         const void *ps[3] = {(const void *)k_ind_pcg_shared<8>, (const void *)k_ind_pcg_shared<16>,
                              (const void *)k_ind_pcg_shared<32>};
         size_t room = prop.sharedMemPerBlockOptin;
@@ -2270,7 +2269,7 @@ static bool solve_pipelined(const Ctx &c) {
 }
 static PcgShape solve_shared(const Ctx &c) {
     if (c.precision != SMD_PREC_MIXED || !solve_pipelined(c)) return PcgShape{};
-    return pcg_shared_shape(c.nmol, c.ind_cap, c.ps_sms, c.ps_smem);
+    return pcg_shared_shape(c.nmol, c.ind_cap, c.sms, c.ps_smem);
 }
 
 int solve_grid(const Ctx &c) {

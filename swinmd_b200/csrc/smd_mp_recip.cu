@@ -19,16 +19,20 @@
 //   torque  2c [ A (mu_i x k) - 2 B (k x Q_i k) ]
 // (permanent terms alone: drop the p terms).
 //
-// Kernels: partial structure factors over (k tile x site chunk) blocks with
-// each chunk's site data staged in shared memory; a fixed-order reduction
-// over chunks giving S(k), the energies and the long virial; one per-site
-// pass for forces and torques with the k data staged in shared memory.  In
-// a time step all six sums come from one pass after the dipole solve and
-// one force pass serves the permanent and induced terms.
-//   FP64 path: a = k.r in FP64 as the reference computes it, FP64 arithmetic.
-//   FP32 path: a is the exact 32-bit integer phase n.(box fractions), sine and
-//   cosine from sincospif; the per-(site, k) arithmetic is FP32 with the
-//   running sums moved into FP64 after every tile of 64-128 terms.
+// Kernels.  Both terms of a step (after the dipole solve) and the permanent one
+// alone go by column products: sums over (column group x site chunk) blocks,
+// a reduction that forms the energies, the virial and the force coefficients,
+// and one per-site pass for forces and torques (below).  FP32 path: exact 32-bit
+// integer phases n.(box fractions), FP32 products, FP64 across chunks and
+// column groups; FP64 path: 64-bit phases, all FP64.  The induced term alone
+// takes its sums by runs of four k and its forces k by k.
+//
+// The general form serves k sets past the tables (|n| > 31) and the reference's
+// forms: partial structure factors over (k tile x site chunk) blocks, a
+// fixed-order reduction over chunks with the energies and the virial, one
+// per-site pass; one sine and cosine per (site, k), of k.r in FP64 as the
+// reference computes it, or of the integer phase (sincospif) with FP32
+// arithmetic and running sums moved into FP64 after every tile of 64-128 terms.
 #include <algorithm>
 #include <cuda_pipeline.h>
 #include <type_traits>
@@ -511,7 +515,7 @@ __global__ void __launch_bounds__(256) k_rforce_f(int n, int nk, const double4 *
 }
 
 // ---------------------------------------------------------------------------
-// FP32 passes of the mixed path
+// Column passes
 // ---------------------------------------------------------------------------
 // The k list is stored column by column: nx, then ny, then nz ascending by
 // one within a column.  The box is orthorhombic, so kx and ky are fixed
@@ -557,12 +561,12 @@ template <typename T> struct ColT;
 template <> struct ColT<float> {
     using T2 = float2;
     using T4 = float4;
-    static constexpr int SUM_THREADS = 128, SUM_SITES = 128, F_THREADS = 256;
+    static constexpr int SUM_THREADS = 128, SUM_SITES = 128;
 };
 template <> struct ColT<double> {
     using T2 = double2;
     using T4 = double4;
-    static constexpr int SUM_THREADS = 128, SUM_SITES = 64, F_THREADS = 128;
+    static constexpr int SUM_THREADS = 128, SUM_SITES = 64;
 };
 __device__ __forceinline__ float tfma(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double tfma(double a, double b, double c) { return fma(a, b, c); }
@@ -643,7 +647,7 @@ __global__ void k_pack_srec_d(int n, const double4 *pos4, const double *tq, cons
     o[3] = make_double4(pind ? pind[2 * N + i] : 0.0, 0.0, 0.0, 0.0);
 }
 
-// MODE 0: permanent sums (slots 0-3); 1: induced sums (4-5); 2: all six.
+// MODE 0: permanent sums (slots 0-3); 1: induced sums (4-5).
 // kseg[s] = (first k, count, nx | ny << 16, first nz)
 template <typename T, int MODE, int SEG>
 __global__ void __launch_bounds__(ColT<T>::SUM_THREADS) k_rsk_seg(int n, int nk, int nseg, int nt, int row,
@@ -654,7 +658,7 @@ __global__ void __launch_bounds__(ColT<T>::SUM_THREADS) k_rsk_seg(int n, int nk,
     using T2 = typename ColT<T>::T2;
     using T4 = typename ColT<T>::T4;
     constexpr int THREADS = ColT<T>::SUM_THREADS, SITES = ColT<T>::SUM_SITES;
-    constexpr bool PERM = MODE != 1, IND = MODE != 0;
+    constexpr bool PERM = MODE == 0, IND = MODE == 1;
     extern __shared__ float4 s_dyn4[];
     T4 *s_v = (T4 *)s_dyn4;                          // [SITES][4]
     T2 *s_tab = (T2 *)(s_v + 4 * SITES);             // [SITES][row]
@@ -1258,15 +1262,6 @@ int blocks_per_sm(const void *kernel, int threads, size_t smem = 0) {
     }
     return per_sm;
 }
-int sm_count() {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 1;
-    }
-    return sms;
-}
 }  // namespace
 
 // nz entries per column (whole items of the sums pass) for nz <= nmax
@@ -1388,7 +1383,7 @@ int mp_recip_prepare(Ctx &c) {
         if (!put(&R.mgrp[q], grp) || !put(&R.mitem[q], item)) return SMD_ERR_CUDA;
         const void *kern = q == 0 ? (const void *)k_col_sums<float, true> : (const void *)k_col_sums<double, true>;
         const size_t sm = q == 0 ? col_sums_smem<float>(row, true) : col_sums_smem<double>(row, true);
-        const int chunk = col_chunk(c.n, R.mblk[q], sm_count() * blocks_per_sm(kern, CS_ITEMS, sm));
+        const int chunk = col_chunk(c.n, R.mblk[q], c.sms * blocks_per_sm(kern, CS_ITEMS, sm));
         const size_t bytes = sizeof(double) * 8 * NZ * item.size();   // of a row of partial sums
         R.mchunk[q] = chunk;
         R.mrows[q] = col_rows((c.n + chunk - 1) / chunk, bytes);
@@ -1423,8 +1418,8 @@ RecipBufs bufs(Ctx &c) {
 
 // site chunks of the partial sums: enough blocks for one full wave of the
 // device (at most MK_CHUNKS, the partial buffer's size)
-int chunks_for(const void *kernel, int kblocks) {
-    const int ch = sm_count() * blocks_per_sm(kernel, MK_THREADS) / (kblocks > 0 ? kblocks : 1);
+int chunks_for(const Ctx &c, const void *kernel, int kblocks) {
+    const int ch = c.sms * blocks_per_sm(kernel, MK_THREADS) / (kblocks > 0 ? kblocks : 1);
     return ch < 1 ? 1 : (ch > MK_CHUNKS ? MK_CHUNKS : ch);
 }
 
@@ -1458,7 +1453,7 @@ int column_sums(Ctx &c, double *partial) {
     constexpr int TH = ColT<T>::SUM_THREADS;
     const int kbt = (c.rc.nseg + TH - 1) / TH;
     const size_t sm = tsum_smem<T>(row);
-    const int ch = sm_count() * blocks_per_sm((const void *)k_rsk_seg<T, MODE, TS_SEG>, TH, sm) / kbt;
+    const int ch = c.sms * blocks_per_sm((const void *)k_rsk_seg<T, MODE, TS_SEG>, TH, sm) / kbt;
     const int nch = ch < 1 ? 1 : (ch > MK_CHUNKS ? MK_CHUNKS : ch);
     k_rsk_seg<T, MODE, TS_SEG><<<dim3(kbt, nch), TH, sm, c.stream>>>(c.n, nk, c.rc.nseg, nt, row, c.rc.kseg,
                                                                      c.rc.kvec, stab, ssv, partial);
@@ -1470,18 +1465,18 @@ void sums(Ctx &c, int slot_e, int slot_e2 = -1) {
     const int nk = c.rc.nk;
     RecipBufs B = bufs(c);
     const int kb = (nk + MK_THREADS - 1) / MK_THREADS;
-    int nch;
-    if (MODE != 2 && c.precision == SMD_PREC_MIXED && column_passes(c)) {
-        nch = column_sums<float, MODE == 2 ? 0 : MODE>(c, B.partial);
-    } else if (c.precision == SMD_PREC_MIXED) {
-        nch = chunks_for((const void *)k_rsk_partial_f<MODE>, kb);
+    int nch = 0;
+    if constexpr (MODE != 2) {   // all six sums only in the general form
+        if (column_passes(c) && c.precision == SMD_PREC_MIXED) nch = column_sums<float, MODE>(c, B.partial);
+        else if (column_passes(c) && !c.reference_forms) nch = column_sums<double, MODE>(c, B.partial);
+    }
+    if (nch == 0 && c.precision == SMD_PREC_MIXED) {
+        nch = chunks_for(c, (const void *)k_rsk_partial_f<MODE>, kb);
         k_rsk_partial_f<MODE><<<dim3(kb, nch), MK_THREADS, 0, c.stream>>>(c.n, nk, c.pos4, c.fixq, c.rc.kn,
                                                                           c.rc.kvec, c.type_q, c.mu, c.qd, c.pind,
                                                                           B.partial);
-    } else if (MODE != 2 && column_passes(c) && !c.reference_forms) {
-        nch = column_sums<double, MODE == 2 ? 0 : MODE>(c, B.partial);
-    } else {
-        nch = chunks_for((const void *)k_rsk_partial<double, MODE>, kb);
+    } else if (nch == 0) {
+        nch = chunks_for(c, (const void *)k_rsk_partial<double, MODE>, kb);
         k_rsk_partial<double, MODE><<<dim3(kb, nch), MK_THREADS, 0, c.stream>>>(c.n, nk, c.pos4, c.fixq, c.rc.kn,
                                                                                c.rc.kvec, c.type_q, c.mu, c.qd,
                                                                                c.pind, B.partial);
@@ -1494,8 +1489,8 @@ void sums(Ctx &c, int slot_e, int slot_e2 = -1) {
 }
 
 // k ranges of the force pass: site blocks x k ranges fill about one wave
-int ksplit_for(const void *kernel, int sblocks, int nk) {
-    const int ks = sm_count() * blocks_per_sm(kernel, 256) / (sblocks > 0 ? sblocks : 1);
+int ksplit_for(const Ctx &c, const void *kernel, int sblocks, int nk) {
+    const int ks = c.sms * blocks_per_sm(kernel, 256) / (sblocks > 0 ? sblocks : 1);
     const int tiles = (nk + FK_TILE - 1) / FK_TILE;
     return ks < 1 ? 1 : (ks > tiles ? tiles : ks);
 }
@@ -1527,7 +1522,7 @@ void column_terms(Ctx &c, int slot_e, int slot_e2) {
     // column ranges of the force pass: about one wave of blocks, at least
     // eight columns each (a range starts with a sine and cosine)
     const int nb = (c.n + CF_THREADS - 1) / CF_THREADS;
-    const int ranges = std::max(1, std::min(R.ncol / 8, 148 * 4 / nb));
+    const int ranges = std::max(1, std::min(R.ncol / 8, c.sms * 4 / nb));
     auto force = [&](auto nzm) {
         const size_t sm = ((size_t)CF_COLS * zn + decltype(nzm)::value) * sizeof(T4);
         k_col_force<T, IND, decltype(nzm)::value><<<dim3(nb, ranges), CF_THREADS, sm, c.stream>>>(
@@ -1548,18 +1543,18 @@ void forces(Ctx &c) {
     const int nb = (int)(((long long)c.n * F_TPS + 255) / 256);
     if (c.precision == SMD_PREC_MIXED) {
         if (PERM) {
-            const int ks = ksplit_for((const void *)k_rforce_f<IND>, nb, nk);
+            const int ks = ksplit_for(c, (const void *)k_rforce_f<IND>, nb, nk);
             k_rforce_f<IND><<<dim3(nb, ks), 256, 0, c.stream>>>(c.n, nk, c.pos4, c.fixq, c.rc.kn, c.rc.kvec,
                                                                 c.rc.kcoef, B.sk, c.type_q, c.mu, c.qd, c.pind,
                                                                 c.frc, c.trq);
         } else {
-            const int ks = ksplit_for((const void *)k_rforce<float, PERM, IND>, nb, nk);
+            const int ks = ksplit_for(c, (const void *)k_rforce<float, PERM, IND>, nb, nk);
             k_rforce<float, PERM, IND><<<dim3(nb, ks), 256, 0, c.stream>>>(c.n, nk, c.pos4, c.fixq, c.rc.kn,
                                                                           c.rc.kvec, c.rc.kcoef, B.sk, c.type_q,
                                                                           c.mu, c.qd, c.pind, c.frc, c.trq);
         }
     } else {
-        const int ks = ksplit_for((const void *)k_rforce<double, PERM, IND>, nb, nk);
+        const int ks = ksplit_for(c, (const void *)k_rforce<double, PERM, IND>, nb, nk);
         k_rforce<double, PERM, IND><<<dim3(nb, ks), 256, 0, c.stream>>>(c.n, nk, c.pos4, c.fixq, c.rc.kn,
                                                                        c.rc.kvec, c.rc.kcoef, B.sk, c.type_q, c.mu,
                                                                        c.qd, c.pind, c.frc, c.trq);
@@ -1588,8 +1583,8 @@ void launch_ind_long(Ctx &c) {
     forces<false, true>(c);
 }
 
-// Both reciprocal terms of a time step, after the dipole solve: one pass for
-// all six structure factors, one force pass
+// Both reciprocal terms of a time step, after the dipole solve: one sums pass and
+// one force pass for the permanent and induced terms
 void launch_polar_long(Ctx &c) {
     if (c.rc.nk == 0) return;
     if (column_passes(c) && c.precision == SMD_PREC_MIXED) {

@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(NHC_BLOCK) k_nhc_second(NhcArgs a) {
             part[Q_MC + 6] += f.x * rz; part[Q_MC + 7] += f.y * rz; part[Q_MC + 8] += f.z * rz;
         }
     }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int w = threadIdx.x >> 5;
     warp_sum_many<NQ>(part, s_part[w]);
     __syncthreads();
     if (threadIdx.x < NQ) {

@@ -418,8 +418,8 @@ void launch_nlist(Ctx &c, bool force_rebuild) {
     a.le = le;
     a.dbox = dbox;
     // blocks loop over the groups, so that a step without a rebuild launches
-    // no more than the device holds at once
-    const int groups = (c.n + NB_SITES - 1) / NB_SITES + c.grid.ncell, nb = groups < 148 * 6 ? groups : 148 * 6;
+    // little more than the device holds at once (five a multiprocessor)
+    const int groups = (c.n + NB_SITES - 1) / NB_SITES + c.grid.ncell, nb = groups < c.sms * 6 ? groups : c.sms * 6;
     if (a.le)
         k_build<true><<<nb, NB_SITES * 32, 0, c.stream>>>(a);
     else

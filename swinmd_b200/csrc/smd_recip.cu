@@ -407,16 +407,12 @@ static int ew_alloc(Ctx &c, int ncap, int nxm, int nym, int mmax) {
         *p = nullptr;
         return cudaMalloc((void **)p, (cnt ? cnt : 1) * sizeof(**p)) == cudaSuccess;
     };
-    int dev = 0, sms = 1;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return SMD_ERR_CUDA;
     r.ew_cap = ncap; r.ew_nx = nxm + 1; r.ew_ny = nym + 1;
     r.ew_nzt = ew_nzt(mmax);
     r.ew_nch = (mmax + r.ew_nzt) / r.ew_nzt;
     const int gx = (ncap * r.ew_nch + ES_THREADS - 1) / ES_THREADS;
     // site chunks: about two blocks of the sums pass per SM
-    r.ew_chunks = std::max(1, std::min(sms, 2 * sms / std::max(gx, 1)));
+    r.ew_chunks = std::max(1, std::min(c.sms, 2 * c.sms / std::max(gx, 1)));
     const size_t slots = (size_t)r.ew_nch * r.ew_nzt * ncap;
     if (!realloc(&r.ew_col, ncap) || !realloc(&r.ew_ncol, 1) || !realloc(&r.ew_coef, slots) ||
         !realloc(&r.ew_part, slots * 4 * r.ew_chunks + ew_totals_size(r)))
@@ -542,11 +538,11 @@ static void launch_columns(Ctx &c, EwArgs a) {
     double *tot = r.ew_part + (size_t)nzp * r.ew_cap * 4 * r.ew_chunks;
     k_ew_reduce<<<dim3((r.ew_cap + ER_COLS - 1) / ER_COLS, nzp), ER_COLS * ER_ROWS, 0, c.stream>>>(
         a, nzp, NZT, chunks, r.ew_part, r.ew_coef, tot);
-    // column ranges of the force pass (blocks of a cluster): about six blocks
-    // per SM, at least four columns each
+    // column ranges of the force pass (blocks of a cluster): at most eight
+    // blocks a multiprocessor, at least four columns each
     const int nb = (c.n + EF_THREADS - 1) / EF_THREADS;
     int ranges = 8;
-    while (ranges > 1 && (ranges * nb > 148 * 8 || ranges * 4 > r.ew_cap)) ranges /= 2;
+    while (ranges > 1 && (ranges * nb > c.sms * 8 || ranges * 4 > r.ew_cap)) ranges /= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nb + 1, ranges);   // the last column of blocks: the totals
     cfg.blockDim = dim3(EF_THREADS);
