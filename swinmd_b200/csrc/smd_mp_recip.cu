@@ -35,6 +35,7 @@
 // arithmetic and running sums moved into FP64 after every tile of 64-128 terms.
 #include <algorithm>
 #include <cuda_pipeline.h>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 #include "smd_ctx.cuh"
@@ -1245,8 +1246,11 @@ size_t tsum_smem(int row) {
     return (size_t)ColT<T>::SUM_SITES * (4 * sizeof(typename ColT<T>::T4) + row * sizeof(typename ColT<T>::T2));
 }
 namespace {
-// resident blocks per SM of each kernel, looked up once per kernel
+// resident blocks per SM of each kernel, looked up once per kernel (contexts
+// may be set up by several threads)
 int blocks_per_sm(const void *kernel, int threads, size_t smem = 0) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
     static const void *keys[32];
     static size_t smems[32];
     static int vals[32], count = 0;
