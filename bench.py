@@ -768,19 +768,28 @@ def main():
             "achieved": flops / t / 1e12, "peak": fp32_peak, "unit": "TFLOP/s",
             "frac": flops / t / 1e12 / fp32_peak, "alg_flops_per_launch": flops, "row_entries": entries,
             "traffic": 17.7e6, "ms": stage_ms["ind_real"],
-            "note": "half of the work is FP64 (nominal FP64 rate 37.2 TFLOP/s); ncu: FP64 pipe 33%, FMA 28%"}
-        # (3) the PCG kernel: every product streams the FP32 tensor rows
-        # (4 B partner + 16 B coefficients per entry) and gathers the packed
-        # vector (16 B per entry); iterations + 1 products per solve
+            "note": "half of the work is FP64 (nominal FP64 rate 37.2 TFLOP/s); ncu: FP64 pipe 35%, FMA 29%, XU 39%"}
+        # (3) the PCG kernel, by the bytes that a block reads from L2 or beyond,
+        # iterations + 1 products per solve: per product the FP32 tensor rows
+        # (4 B partner + 16 B coefficients per entry) and the vector, either
+        # gathered (16 B per entry) or copied whole into every block's shared
+        # memory (12 B a site); row slots held there are read once per solve
         products = fast["solver_iterations"] + 1
-        nbytes = products * entries * (4 + 16 + 16)
+        lay = np.zeros(3, np.int32)
+        L.check(ens.ctx, ens.lib.smd_solver_layout(ens.ctx, L.iptr(lay)))
+        form, blocks, slots = (int(x) for x in lay)
+        held = n * min(float(slots), entries / n)
+        nbytes = (products * ((entries - held) * (4 + 16) + blocks * 12.0 * n) + held * (4 + 16) if form == 2
+                  else products * entries * (4 + 16 + 16))
         t = stage_ms["pcg"] * 1e-3
         rooflines["pcg"] = {
-            "bound": "hbm", "kernel": "k_ind_pcg_shared (pipelined PCG, molecule blocks)",
+            "bound": "l2", "kernel": ("k_ind_cg", "k_ind_pcg_pipe", "k_ind_pcg_shared")[form],
             "achieved": nbytes / t / 1e9, "peak": hbm_peak,
             "unit": "GB/s", "frac": nbytes / t / 1e9 / hbm_peak, "alg_bytes_per_launch": nbytes,
-            "products": products, "traffic": None, "ms": stage_ms["pcg"],
-            "note": "the gathered vector and part of the rows sit in shared memory, the rest comes from L2 (126 MB)"}
+            "products": products, "blocks": blocks, "held_slots_per_site": slots, "traffic": 93e6,
+            "ms": stage_ms["pcg"],
+            "note": "bytes from L2; no L2 rate is measured, the HBM copy rate stands in for the peak; grid barriers "
+                    "between the products"}
         # the dominant kernel: the largest device time of one kernel (the
         # reciprocal figure covers two kernels)
         rooflines["polar_recip"]["kernels"] = 2
@@ -795,7 +804,7 @@ def main():
     roofline.update(peak_source=f"HBM: hbm_gbs of MEASURED_PEAKS.json ({peak_src}); FP32: nominal SIMT rate "
                                 "148 SMs x 128 lanes x 2 at sm_max_mhz (the file has no FP32 figure)",
                     dominant_stage=dom,
-                    traffic_source="ncu --set full captures of the polwater4096 step (profiles/)")
+                    traffic_source="DRAM bytes of one launch under ncu, polwater4096 (profiles/step_kernels.md)")
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline and polar:

@@ -297,6 +297,11 @@ int smd_set_wait_limit(smd_ctx *ctx, double seconds);
 int smd_test_skip_arrival(smd_ctx *ctx, int block);
 /* Solver statistics of the last solve: iterations and final RMS change. */
 int smd_solver_stats(smd_ctx *ctx, int *iterations, double *rms_change);
+/* The dipole solve that the present settings choose: layout[0] its form (0
+ * single-reduction PCG, 1 pipelined, 2 pipelined with the vector in shared
+ * memory), layout[1] its blocks, layout[2] the slots of each site's tensor row
+ * that form 2 holds in shared memory (0 otherwise). */
+int smd_solver_layout(smd_ctx *ctx, int32_t *layout);
 /* RMS change of the dipoles at each iteration of the last solve (the
  * quantity the tolerance is tested on), up to 64 iterations: rms[k] for
  * k < min(count, cap).  The first entry measures how far the start was. */

@@ -146,6 +146,7 @@ SIGNATURES = {
     "smd_set_solver": (ctypes.c_int, [_P, ctypes.c_double, ctypes.c_int, ctypes.c_int]),
     "smd_set_preconditioner": (ctypes.c_int, [_P, ctypes.c_int]),
     "smd_solver_stats": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int), _D]),
+    "smd_solver_layout": (ctypes.c_int, [_P, _I]),
     "smd_solver_trace": (ctypes.c_int, [_P, _D, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]),
     "smd_set_wait_limit": (ctypes.c_int, [_P, ctypes.c_double]),
     "smd_test_skip_arrival": (ctypes.c_int, [_P, ctypes.c_int]),

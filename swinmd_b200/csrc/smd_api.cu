@@ -982,6 +982,12 @@ int smd_solver_stats(smd_ctx *x, int *iterations, double *rms_change) {
     return SMD_OK;
 }
 
+int smd_solver_layout(smd_ctx *x, int32_t *layout) {
+    if (!x || !layout || !x->c.cgs) return fail(x, SMD_ERR_ARG, "smd_solver_layout: no dipole solver");
+    solve_layout(x->c, layout);
+    return SMD_OK;
+}
+
 int smd_solver_trace(smd_ctx *x, double *rms, int cap, int *count) {
     if (!x || !x->c.cgs || !count || (cap > 0 && !rms)) return fail(x, SMD_ERR_ARG, "smd_solver_trace: bad arguments");
     double s[CG_SCAL + CG_TRACE];

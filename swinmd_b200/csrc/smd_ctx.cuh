@@ -487,6 +487,7 @@ __host__ __device__ inline void acc_energies(const long long *acc, double e_lrc,
 void launch_buff(Ctx &c);
 int setup_cg(Ctx &c);
 int solve_grid(const Ctx &c);   // blocks of the dipole solve that the present settings choose
+void solve_layout(const Ctx &c, int32_t *layout);   // its form, blocks and held slots (smd_solver_layout)
 int recip_nk(Ctx &c, int *nk);
 int ensure_ind_rows(Ctx &c);
 // dipole-guess network (smd_mlp.cu)

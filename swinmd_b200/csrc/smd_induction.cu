@@ -2277,6 +2277,13 @@ int solve_grid(const Ctx &c) {
     return s.threads > 0 ? s.blocks : (solve_pipelined(c) ? c.pp_blocks : c.cg_blocks);
 }
 
+void solve_layout(const Ctx &c, int32_t *layout) {
+    const PcgShape s = solve_shared(c);
+    layout[0] = s.threads > 0 ? 2 : (solve_pipelined(c) ? 1 : 0);
+    layout[1] = solve_grid(c);
+    layout[2] = s.threads > 0 ? s.slots : 0;
+}
+
 void launch_ind_cg(Ctx &c) {
     IndArgs a = ind_args(c);
     const bool f32 = c.precision == SMD_PREC_MIXED;
