@@ -852,12 +852,13 @@ __device__ __forceinline__ void add_moments(int n, int i, const double4 *pos4, c
 // column's X^nx Y^ny follows from the one before along ny in FP64 and is
 // rounded once.  The moments fold into M1..M3 as below.
 //
-// FMA issue and shared-memory reads bound both (FMA pipe 55 to 58 % busy).
-// 12 288 sites x 12 151 k in FP32, against one thread per run of 4 k (six
-// sums, 27 instructions a (site, k)) and per site walking k by k (26
-// instructions): sums 166 -> 105, reduction 4 -> 9, forces 159 -> 79 us; 3993
-// sites, FP64: 80 -> 36 and 41 -> 21 us.  The sums with 3, 4, 5, 6 and 9 nz an
-// item measured 106, 107, 105, 105 and 119 us.
+// FMA issue and shared-memory reads bound the sums (FMA pipe 56 % busy, L1 and
+// shared memory 66 %), issue the forces (79 %, FMA pipe 59 %).  12 288 sites x
+// 12 151 k in FP32, against one thread per run of 4 k (six sums, 27 instructions
+// a (site, k)) and per site walking k by k (26 instructions): sums 166 -> 107,
+// reduction 4 -> 9, forces 159 -> 76 us; 3993 sites, FP64: 80 -> 32 and 41 -> 21
+// us.  The sums with 3, 4, 5, 6 and 9 nz an item measured 106, 107, 105, 105 and
+// 119 us (FP32 block sums).
 template <typename T> struct ColP;
 template <> struct ColP<float> { static constexpr int NZ = 5; };
 template <> struct ColP<double> { static constexpr int NZ = 2; };
@@ -1280,7 +1281,7 @@ size_t col_sums_smem(int row, bool ind) {
 // sites per block of the sums pass: whole sub-tiles, at most CS_CHUNK, such
 // that the blocks' waves (resident blocks at a time) leave least idle; a
 // block's own start counts as half a sub-tile.  12 288 sites, 12 column
-// groups, 444 resident: 96 sites in 3.5 waves against 128 in 2.6
+// groups, 444 resident: 112 sites in 3.0 waves against 96 in 3.5 and 128 in 2.6
 int col_chunk(int n, int nblk, int resident) {
     int best = CS_SUB;
     long long least = 1LL << 62;

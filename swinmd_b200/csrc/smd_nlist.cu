@@ -235,7 +235,9 @@ __global__ void __launch_bounds__(NB_SITES * 32, 5) k_build(BuildArgs a) {
     if (a.group) {
         far = a.flags[5];
     } else {
-        for (int j = threadIdx.x; j < a.n; j += NB_SITES * 32) far = far || far_out(a.pos4[j], box);
+        // eight loads of a thread in flight
+#pragma unroll 8
+        for (int j = threadIdx.x; j < a.n; j += NB_SITES * 32) far |= far_out(a.pos4[j], box);
         far = __syncthreads_or(far);
     }
     for (int gi = blockIdx.x; gi < ngroup; gi += gridDim.x) {

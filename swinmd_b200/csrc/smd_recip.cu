@@ -150,8 +150,9 @@ __global__ void __launch_bounds__(LC_THREADS) k_le_columns(int nxm, int nyr, int
 // column (items ordered nz range by nz range, so that a warp's Z loads are
 // broadcasts and its Y loads consecutive) and runs over the block's chunk of
 // sites, whose factor powers stand in shared memory tile by tile.  The 4 NZT
-// running sums in registers give 4 NZT FMAs per 2 + NZT shared loads; the
-// bound is FP64 issue (8000 ions, 2094 k: 34 M FMAs, 2 us).
+// running sums in registers give 4 NZT FMAs per 2 + NZT shared loads.  8000
+// ions, 2094 k: 13.8 us, of which FP64 issue would take 2 (34 M FMAs; pipe 27 %
+// busy): waits for shared memory and the tiles' barriers with few warps a block.
 template <int NZT>
 __global__ void __launch_bounds__(ES_THREADS) k_ew_sums(EwArgs a, double *part) {
     extern __shared__ double2 s_tab[];   // [tile][row]
@@ -303,10 +304,11 @@ __device__ __forceinline__ void ew_totals(int nzp, int gx, int nb, const double 
 
 // Per-site force.  The blocks of a cluster (along y) split the columns, so
 // that a few thousand sites fill the device; their partial forces meet in
-// shared memory over the cluster and enter the fixed-point sum once.  A thread keeps its site's Z^nz and nz Z^nz of one nz range in
-// registers, so a column costs two broadcast shared loads and eight FMAs per
-// nz; the column's X^nx Y^ny follows from the one before along ny.  FP64
-// issue bounds it (8000 ions, 2094 k: 67 M FMAs, 4 us).
+// shared memory over the cluster and enter the fixed-point sum once.  A thread
+// keeps its site's Z^nz and nz Z^nz of one nz range in registers, so a column costs two broadcast shared loads and eight FMAs per
+// nz; the column's X^nx Y^ny follows from the one before along ny.  8000 ions,
+// 2094 k: 22.5 us, of which FP64 issue would take 4 (67 M FMAs; pipe 32 % busy):
+// the dependent FP64 chains of a column and the barriers between groups.
 template <int NZT>
 __global__ void __launch_bounds__(EF_THREADS) k_ew_force(EwArgs a, const double4 *coef, long long *frc, const double *tot,
                                                          long long *acc) {
